@@ -201,10 +201,10 @@ def test_grouped_products_activation_and_weighted_sum(ops, dt, tile):
 
 @pytest.mark.parametrize("n_out, K", [(264, 72), (40, 200), (515, 64)])
 @pytest.mark.parametrize("out32", [True, False])
-def test_grouped_products_of_paired_blocks(ops, n_out, K, out32):
-    """128-row tiles run on pairs of blocks that walk through several items each: experts without rows, with
-    the row counts around a stored chunk (16) and a tile (128), and a last block of few features.  The sums
-    hold K exact products in 32 bits: within K 2^-22 of the largest sum of magnitudes."""
+def test_grouped_products_of_128_row_tiles(ops, n_out, K, out32):
+    """128-row tiles alone: experts without rows, with the row counts around a stored chunk (16) and a tile
+    (128), and a last block of few features.  The sums hold K exact products in 32 bits: within K 2^-22 of
+    the largest sum of magnitudes."""
     g = torch.Generator().manual_seed(n_out)
     counts = [0, 1, 15, 16, 17, 127, 128, 129, 300, 0] + [33] * 70
     E, rows = len(counts), sum(counts)
@@ -226,6 +226,49 @@ def test_grouped_products_of_paired_blocks(ops, n_out, K, out32):
         bound = (x.abs() @ we.abs().T) * (K * 2.0 ** -22 + (0 if out32 else 2.0 ** -8))
         assert ((out[first[e]:first[e] + c].double().cpu() - x @ we.T).abs() <= bound).all(), e
     assert status.item() == 0
+
+
+@pytest.mark.parametrize("tile, n", [(16, 90), (64, 500), (128, 2048)])
+def test_routed_passes_follow_one_another_without_a_wait(ops, tile, n):
+    """Plan, gathered rows, both grouped products (the activation in the first one's epilogue) and the weighted
+    sum, pass after pass with nothing waited for between them and a new plan in every pass: the first pass's
+    result each time, and no wait on a barrier that gave up."""
+    g = torch.Generator().manual_seed(tile)
+    D, F, E, top = 264, 136, 32, 4
+    h = torch.randn(n, D, generator=g).bfloat16().to(DEV)
+    wgu = (0.1 * torch.randn(E, 2 * F, D, generator=g)).bfloat16().to(DEV)
+    wd = (0.1 * torch.randn(E, D, F, generator=g)).bfloat16().to(DEV)
+    choice = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)]).to(torch.int32)
+    filled = torch.bincount(choice.reshape(-1).long(), minlength=E).to(torch.int32).to(DEV)
+    choice, weight = choice.reshape(-1).to(DEV), torch.rand(n * top, generator=g).to(DEV)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    pairs, mt = n * top, ops.routed_max_tiles(n * top, E, tile)
+    counts, first = torch.zeros(E, **i32), torch.zeros(E + 1, **i32)
+    pair_row, row_token = torch.zeros(pairs, **i32), torch.zeros(pairs, **i32)
+    plan = (first, torch.zeros(mt, **i32), torch.zeros(mt, **i32), torch.zeros(1, **i32), mt)
+    rows = torch.empty(pairs, D, dtype=torch.bfloat16, device=DEV)
+    act = torch.empty(pairs, F, dtype=torch.bfloat16, device=DEV)
+    y, status = torch.empty(pairs, D, device=DEV), torch.zeros(1, **i32)
+    outs = torch.zeros(40, n, D, device=DEV)
+    for out in outs:
+        counts.copy_(filled)
+        ops.route_plan(counts, choice, pairs, top, E, first, pair_row, row_token, *plan[1:4], tile_rows=tile)
+        ops.gather_rows(h, row_token, rows)
+        ops.gemm_grouped_tc(rows, wgu, act, *plan, tile, status, glu=(1.702, 1.1, 1.0))
+        ops.gemm_grouped_tc(act, wd, y, *plan, tile, status)
+        ops.routed_combine(out, y, pair_row, weight, top, accumulate=False)
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    hc, ref = h.float().cpu(), torch.zeros(n, D)
+    c, w = choice.cpu().view(n, top).long(), weight.cpu().view(n, top)
+    for e in range(E):
+        t, j = (c == e).nonzero(as_tuple=True)
+        gu = hc[t] @ wgu[e].float().cpu().T
+        gg, uu = torch.clamp(gu[:, :F], max=1.1), torch.clamp(gu[:, F:], -1.1, 1.1)
+        a = (gg * torch.sigmoid(1.702 * gg) * (uu + 1.0)).bfloat16().float()
+        ref.index_add_(0, t, w[t, j, None] * (a @ wd[e].float().cpu().T))
+    assert (outs[0].cpu() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item()
+    assert all(torch.equal(out, outs[0]) for out in outs[1:])
 
 
 @pytest.mark.parametrize("dt, eps", HALF)

@@ -1145,239 +1145,6 @@ static int two_sm_token_tile(int M, int n_out, int splits) {
   return best_bt;
 }
 
-// ===========================================================================
-// The grouped product of many rows on pairs of SMs: gemm_2sm_kernel's roles, barriers and double
-// accumulators, persistent over (tile of the plan, 256 features).  A pair takes 256 features x 128 rows of one
-// expert; with NACC == 2 it holds gate and up of the same 256 features.  Rows leave through TMA in chunks
-// of 16; an expert's last, shorter chunk (TMA would run on into the next expert's rows) is stored by the
-// threads.  The epilogue of one item runs under the products of the next, which the single-SM form above (a
-// block per tile, one to an SM, its start and its end bare) does not have: 8,192 rows of 32 experts, gate/up
-// of 768 features over 2,048 and down to 2,048: 92 + 59 us there, 73 + 46 here.
-constexpr int GP_BT = 128;
-
-template <int NACC>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS)
-gemm_2sm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
-                        const __grid_constant__ CUtensorMap map_out, int out_tma, void* __restrict__ out,
-                        int out_dtype, int ab_dtype, int N, int K, const int* __restrict__ first_row,
-                        const int* __restrict__ tile_expert, const int* __restrict__ tile_row0,
-                        const int* __restrict__ n_tiles, GluParams glu, int* __restrict__ status) {
-  using Cfg = G2Cfg<GP_BT, NACC>;
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[Cfg::STAGES];
-  __shared__ __align__(8) uint64_t empty_bar[Cfg::STAGES];
-  __shared__ __align__(8) uint64_t acc_full[2];
-  __shared__ __align__(8) uint64_t acc_empty[2];
-  __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag;
-  __shared__ __align__(128) uint8_t epi_smem[2 * 16 * TC_BM * 4];   // two chunks of 16 rows, row-major
-
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const uint32_t rank = __shfl_sync(0xffffffffu, cluster_rank(), 0);
-  const bool leader = rank == 0;
-  const uint32_t tiles_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int n_out = NACC == 2 ? N / 2 : N;
-  const int n_feat = (n_out + 2 * TC_BM - 1) / (2 * TC_BM);
-  const int nkb = (K + TC_BK - 1) / TC_BK;
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-
-  if (threadIdx.x == 0) {
-    abort_flag = 0;
-    for (int s = 0; s < Cfg::STAGES; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), 1);
-      mbar_init(smem_u32(&empty_bar[s]), 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&acc_full[b]), 1);
-      mbar_init(smem_u32(&acc_empty[b]), 2 * (SK_EPI_THREADS / 32));
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  cluster_sync_all();                                        // both blocks' barriers exist
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
-  volatile int* abort_p = &abort_flag;
-  pdl_launch_dependents();
-  pdl_wait();                                                // the plan comes from the previous kernels
-  const int n_items = __shfl_sync(0xffffffffu, *n_tiles, 0) * n_feat;
-
-  if (warp == 0) {
-    // ---------------- TMA producer (warp 0 of each block runs the loop, its lane 0 issues)
-    const uint32_t issue = lane == 0 ? 1u : 0u;
-    int it = 0;
-    bool ok = true;
-    for (int t = pair; t < n_items && ok; t += n_pairs) {
-      const int tile = t / n_feat;
-      const int w_row = __shfl_sync(0xffffffffu, tile_expert[tile], 0) * N + (t - tile * n_feat) * 2 * TC_BM +
-                        (int)rank * TC_BM;
-      const int a_row = __shfl_sync(0xffffffffu, tile_row0[tile], 0) + (int)rank * (GP_BT / 2);
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
-        const int s = it % Cfg::STAGES;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&empty_bar[s]), ((it / Cfg::STAGES) & 1) ^ 1u, abort_p));
-        if (!ok) break;
-        const uint32_t stage = tiles_smem + s * Cfg::STAGE_BYTES;
-        const uint32_t bar0 = map_to_rank(smem_u32(&full_bar[s]), 0);     // the first block's
-        mbar_expect_tx_by(leader ? issue : 0u, smem_u32(&full_bar[s]), 2 * Cfg::STAGE_BYTES);
-        const int kx = kb * TC_BK;
-        tma_load_2d_pair_by(issue, stage, &map_w, kx, w_row, bar0);
-        if (NACC == 2) tma_load_2d_pair_by(issue, stage + Cfg::W_BYTES, &map_w, kx, w_row + n_out, bar0);
-        tma_load_2d_pair_by(issue, stage + NACC * Cfg::W_BYTES, &map_a, kx, a_row, bar0);
-      }
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer: warp 1 of the first block runs the loop, its lane 0 issues for the pair
-    if (leader) {
-      const uint32_t issue = lane == 0 ? 1u : 0u;
-      const uint32_t idesc = umma_idesc(ab_dtype, GP_BT, 2 * TC_BM);
-      bool ok = true;
-      int it = 0, part = 0;
-      for (int t = pair; t < n_items && ok; t += n_pairs, ++part) {
-        const int buf = part & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty[buf]), (((uint32_t)part >> 1) & 1u) ^ 1u, abort_p));
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc_addr = tmem_base + (uint32_t)(buf * Cfg::ACC_STRIDE);
-        for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
-          const int s = it % Cfg::STAGES;
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full_bar[s]), (it / Cfg::STAGES) & 1, abort_p));
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t stage = tiles_smem + s * Cfg::STAGE_BYTES;
-          const uint64_t wdesc = umma_desc_k_sw128(stage);
-          const uint64_t adesc = umma_desc_k_sw128(stage + NACC * Cfg::W_BYTES);
-#pragma unroll
-          for (int k = 0; k < TC_BK / TC_UMMA_K; ++k) {
-            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-            const uint64_t koff = (uint64_t)((k * TC_UMMA_K * 2) >> 4);
-            umma_f16_pair_by(issue, acc_addr, wdesc + koff, adesc + koff, idesc, acc);
-            if (NACC == 2) {
-              const uint64_t w2 = umma_desc_k_sw128(stage + Cfg::W_BYTES);
-              umma_f16_pair_by(issue, acc_addr + GP_BT, w2 + koff, adesc + koff, idesc, acc);
-            }
-          }
-          umma_commit_pair_by(issue, smem_u32(&empty_bar[s]));           // frees the stage in both blocks
-        }
-        if (ok) umma_commit_pair_by(issue, smem_u32(&acc_full[buf]));    // both blocks' epilogues may read
-      }
-    }
-  } else {
-    // ---------------- epilogue warps of both blocks: this block's 128 features
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const int esz = out_dtype == DT_F32 ? 4 : 2;
-    int part = 0, stage_it = 0;
-    for (int t = pair; t < n_items; t += n_pairs, ++part) {
-      const int buf = part & 1;
-      const int tile = t / n_feat;
-      const int x = (t - tile * n_feat) * 2 * TC_BM + (int)rank * TC_BM;
-      const int row0 = tile_row0[tile];
-      const int rows = min(GP_BT, first_row[tile_expert[tile] + 1] - row0);
-      const int f = x + row;
-      const bool issuer = row == 0 && x < n_out;             // (a block whose features lie beyond N copies nothing)
-      const bool got = mbar_wait(smem_u32(&acc_full[buf]), ((uint32_t)part >> 1) & 1u, abort_p);
-      // whether any thread gave up: all of them leave together
-      uint32_t gave_up;
-      asm volatile(
-          "{\n.reg .pred p, q;\nsetp.ne.b32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
-          : "=r"(gave_up) : "r"(got ? 0u : 1u), "n"(SK_EPI_THREADS) : "memory");
-      if (gave_up) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * Cfg::ACC_STRIDE);
-#pragma unroll 1
-      for (int c0 = 0; c0 < rows; c0 += 16) {
-        float v[16];
-        tmem_ld16(taddr + c0, v);
-        if (NACC == 2) {
-          float u[16];
-          tmem_ld16(taddr + GP_BT + c0, u);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = glu_clamped_fast(v[j], u[j], glu);
-        }
-        if (!out_tma || c0 + 16 > rows) {
-          sk_store_chunk(0, out_dtype, out, v, f, row0 + c0, row0 + rows, n_out);
-          continue;
-        }
-        const uint32_t st = smem_u32(epi_smem) + (uint32_t)((stage_it & 1) * 16 * TC_BM * esz);
-        // the copy that read this buffer two chunks ago has read it
-        if (issuer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI_THREADS) : "memory");
-        if (out_dtype == DT_F32) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(st + (uint32_t)((j * TC_BM + row) * 4)), "f"(v[j]) : "memory");
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(st + (uint32_t)((j * TC_BM + row) * 2)),
-                         "h"(bits16_rt(out_dtype, v[j])) : "memory");
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI_THREADS) : "memory");
-        if (issuer) {
-          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
-                       ::"l"(reinterpret_cast<uint64_t>(&map_out)), "r"(st), "r"(x), "r"(row0 + c0) : "memory");
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-        ++stage_it;
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[buf]), 0));
-    }
-    // the copies this thread handed to the copy engine are done before the block ends
-    if (row == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  }
-
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (abort_flag) {
-    if (threadIdx.x == 0) atomicOr(status, ERR_WAIT_TIMEOUT);
-    const unsigned long long t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
-    __syncthreads();
-  }
-  cluster_sync_all();                  // nobody touches the peer's barriers or TMEM after this
-  if (warp == 1) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;"
-                 ::"r"(tmem_base), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
-  }
-}
-
-template <int NACC>
-static int launch_2sm_grouped(const void* A, const void* W, void* out, int out_dtype, int ab_dtype, int rows_total,
-                              int E, int N, int K, const int* first_row, const int* tile_expert, const int* tile_row0,
-                              const int* n_tiles, int max_tiles, const GluParams& glu, int* status,
-                              cudaStream_t stream) {
-  using Cfg = G2Cfg<GP_BT, NACC>;
-  CUtensorMap mw, ma, mo;
-  int rc = make_map(&mw, W, E * N, K, TC_BM, ab_dtype);
-  if (rc) return rc;
-  rc = make_map(&ma, A, rows_total, K, GP_BT / 2, ab_dtype);
-  if (rc) return rc;
-  const int n_out = NACC == 2 ? N / 2 : N, esz = out_dtype == DT_F32 ? 4 : 2;
-  mo = ma;
-  const int out_tma = ((uintptr_t)out & 15) == 0 && ((long long)n_out * esz) % 16 == 0 &&
-                      make_out_map(&mo, out, rows_total, n_out, out_dtype, TC_BM) == 0;
-  const cudaError_t e =
-      cudaFuncSetAttribute(gemm_2sm_grouped_kernel<NACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
-  if (e != cudaSuccess) return (int)e;
-  long long pairs = (long long)max_tiles * ((n_out + 2 * TC_BM - 1) / (2 * TC_BM));
-  if (pairs > sm_count() / 2) pairs = sm_count() / 2;
-  launch_pdl(gemm_2sm_grouped_kernel<NACC>, dim3((unsigned)(2 * pairs)), dim3(TC_THREADS), Cfg::SMEM, stream, mw, ma, mo,
-             out_tma, out, out_dtype, ab_dtype, N, K, first_row, tile_expert, tile_row0, n_tiles, glu, status);
-  YALM_LAUNCH_CHECK();
-  return 0;
-}
-
 }  // namespace yalm
 
 using namespace yalm;
@@ -1480,18 +1247,14 @@ extern "C" int yalm_gemm_grouped_tc(const void* A, const void* W, int ab_dtype, 
     if (tile_rows == 16) YALM_TCG(16, 2);
     if (tile_rows == 32) YALM_TCG(32, 2);
     if (tile_rows == 64) YALM_TCG(64, 2);
-    if (tile_rows == GP_BT)
-      return launch_2sm_grouped<2>(A, W, out, out_dtype, ab_dtype, rows_total, E, N, K, first_row, tile_expert,
-                                   tile_row0, n_tiles, max_tiles, glu, status, stream);
+    if (tile_rows == 128) YALM_TCG(128, 2);
     if (tile_rows == 256) YALM_TCG(256, 2);
     return -2;
   }
   if (tile_rows == 16) YALM_TCG(16, 1);
   if (tile_rows == 32) YALM_TCG(32, 1);
   if (tile_rows == 64) YALM_TCG(64, 1);
-  if (tile_rows == GP_BT)
-    return launch_2sm_grouped<1>(A, W, out, out_dtype, ab_dtype, rows_total, E, N, K, first_row, tile_expert,
-                                 tile_row0, n_tiles, max_tiles, glu, status, stream);
+  if (tile_rows == 128) YALM_TCG(128, 1);
   if (tile_rows == 256) YALM_TCG(256, 1);
   return -2;
 #undef YALM_TCG
