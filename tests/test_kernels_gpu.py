@@ -619,12 +619,13 @@ def test_decode_attention_with_the_rotary_work_inside(ops, H, G, hd, cap, window
 
 
 @pytest.mark.parametrize("shape", [(1, 128, 64), (130, 300, 88), (256, 256, 64), (300, 512, 128),
-                                   (700, 640, 448), (1500, 1152, 320), (2048, 1024, 1024),
+                                   (700, 640, 448), (1500, 1152, 320), (2048, 1024, 1024), (14331, 640, 64),
                                    (512, 9472, 64)])
 @pytest.mark.parametrize("dt, eps", HALF)
 def test_two_sm_matrix_product(ops, shape, dt, eps):
     """gemm_2sm: a cluster of two blocks per 256-feature tile (tcgen05.mma.cta_group::2),
-    every epilogue, sizes that leave the second block of a pair partly or wholly empty.
+    every epilogue, sizes that leave the second block of a pair partly or wholly empty (with 14,331 rows
+    of 640 features such an item follows, in the same pair, one whose stores are still on their way).
     The token tile is 240 wherever its waves over the 74 pairs cost no more than those of
     256 (all shapes but the last: 37 feature tiles x 2 token tiles of 256 are one wave,
     x 3 of 240 would be two)."""

@@ -962,9 +962,10 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // 64 output features; a chunk goes token-major ([16][64] of the 16-bit type) into one
         // of two staging buffers (see the store below)
         const int x = (feat0 + (int)rank * TC_BM) >> 1;
-        const bool issuer = row == 0 && x < (N >> 1);
+        const bool issuer = row == 0;
+        const int cols = x < (N >> 1) ? ncols : 0;           // (nothing to stage beyond N, as below)
 #pragma unroll 1
-        for (int c0 = 0; c0 < ncols; c0 += 16, ++stage_it) {
+        for (int c0 = 0; c0 < cols; c0 += 16, ++stage_it) {
           float v[16];
           tmem_ld16(taddr + c0, v);
           float r[8];
@@ -992,10 +993,13 @@ gemm_2sm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // warp instruction, kept a tile's last epilogue 5-6 us long; tokens beyond M are
         // clipped by the tensor map)
         const int x = feat0 + (int)rank * TC_BM;
-        const bool issuer = row == 0 && x < n_out;           // (a block whose features lie beyond N copies nothing)
+        const bool issuer = row == 0;
+        // A block whose features lie beyond N has nothing to store and stages nothing: it would write
+        // a buffer that the last item's copy may still be reading, and the wait below lets the newest copy run on.
+        const int cols = x < n_out ? ncols : 0;
         const int esz = out_dtype == DT_F32 ? 4 : 2;
 #pragma unroll 1
-        for (int c0 = 0; c0 < ncols; c0 += 16, ++stage_it) {
+        for (int c0 = 0; c0 < cols; c0 += 16, ++stage_it) {
           float v[16];
           tmem_ld16(taddr + c0, v);
           if (mode == 0 && glu.store_act != 0) {
