@@ -994,3 +994,58 @@ def test_tcgen05_attention_with_unrounded_weights(ops, H, G, hd, window, pool, k
         bad = (err > bound).any(-1).nonzero()
         assert not bad.numel(), (lens, int(bad[0]), float(err.max()))
         ops.advance(b, slot_pos)
+
+
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("kind, hd, window, cap, pool, keep", [
+    ("step", 128, 0, 700, 0, 0), ("step", 64, 100, 700, 0, 0), ("cache", 128, 0, 700, 0, 0), ("cache", 64, 90, 700, 0, 0),
+    ("ring", 128, 100, 100, 0, 0), ("ring", 64, 130, 150, 0, 0), ("exact", 128, 0, 700, 0, 0), ("exact", 64, 100, 110, 0, 0),
+    ("exact", 128, 100, 100, 16, 0), ("exact", 64, 100, 700, 0, 70)])
+@pytest.mark.parametrize("dt, eps", HALF)
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_tcgen05_attention_keeps_foreign_rows_out(ops, kind, hd, window, cap, pool, keep, dt, eps, paged, bad):
+    """Infinities and NaN in the next sequence's keys and values, in rows of the cache and of the pooled blocks that
+    a sequence has not written, and in the next slot's rows: the other sequences' bits are those without them."""
+    H, G, n_slots, slots, steps = 4, 2, 5, [2, 0, 3], ([150, 70, 33], [90, 65, 100], [31, 64, 257])
+    pcap = 700 // max(pool, 1) + 1
+    outs = []
+    for value in (0.0, bad):
+        g = torch.Generator().manual_seed(hd + window + cap)
+        fill = lambda c: torch.full((n_slots, G, c, hd), value, device=DEV, dtype=dt)
+        kc, vc, table, pk, pv, ptable = fill(cap), fill(cap), None, fill(pcap), fill(pcap), None
+        if paged:
+            kc, vc, table = _paged(kc, vc, seed=cap)
+            pk, pv, ptable = _paged(pk, pv, seed=cap + 1)
+        slot_pos = torch.zeros(n_slots, dtype=torch.int32, device=DEV)
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        outs.append([])
+        for lens in steps[:1] if kind == "step" else steps:
+            b = B(lens, slots)
+            N, qs = b.n_tokens, b.q_start.tolist()
+            q = torch.randn(N, H * hd, generator=g).to(dt).to(DEV)
+            kv = torch.randn(N, 2, G, hd, generator=g).to(dt).to(DEV)
+            if value:
+                kv[qs[1]:qs[2]] = value                       # the sequence in the middle
+            out = torch.full((N, H * hd), 9.0, device=DEV, dtype=dt)
+            pooled = (pk, pv, pool, pcap, ptable) if pool else None
+            if pool:
+                ops.pool_blocks(kv, kc, vc, b, slot_pos, pk, pv, G, hd, cap, pool, pcap, status, pages=table,
+                                pool_pages=ptable)
+            write = lambda: ops.cache_write(kv, b, kc, vc, slot_pos, G, hd, cap, pages=table)
+            if kind == "step":
+                ops.attention_prefill_tc(q, kv, b, out, H, G, hd, window or None, status)
+            elif kind == "cache":
+                write()
+                ops.attention_prefill_tc_cache(q, kc, vc, b, slot_pos, out, H, G, hd, cap, window or None, status, pages=table)
+            elif kind == "ring":
+                ops.attention_prefill_tc_ring(q, kv, kc, vc, b, slot_pos, out, H, G, hd, cap, window, status, pages=table)
+            else:
+                ops.attention_exact_tc(q, kv, kc, vc, b, slot_pos, out, H, G, hd, cap, window or None, status, pages=table,
+                                       pooled=pooled, keep_first=keep or None)
+            if kind != "cache":
+                write()
+            ops.advance(b, slot_pos)
+            assert status.item() == 0
+            outs[-1] += [out[qs[i]:qs[i + 1]].clone() for i in (0, 2)]
+    for i, (clean, got) in enumerate(zip(*outs)):
+        assert torch.equal(clean, got), (i, int((clean != got).any(-1).nonzero()[0]))

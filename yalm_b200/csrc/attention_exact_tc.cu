@@ -70,6 +70,7 @@ attn_exact_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   extern __shared__ uint8_t xt_smem[];
   __shared__ __align__(8) uint64_t q_full, s_full[2], p_ready[2], pv_done[2];
   __shared__ __align__(8) uint64_t k_full[XT_STAGES], k_empty[XT_STAGES], v_full[XT_STAGES], v_empty[XT_STAGES];
+  __shared__ __align__(8) uint64_t v_landed;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -142,6 +143,7 @@ attn_exact_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       mbar_init(smem_u32(&p_ready[x]), TA_BM);
       mbar_init(smem_u32(&pv_done[x]), 1);
     }
+    mbar_init(smem_u32(&v_landed), 1);
     for (int s = 0; s < XT_STAGES; ++s) {
       mbar_init(smem_u32(&k_full[s]), 1);
       mbar_init(smem_u32(&k_empty[s]), 2);
@@ -164,9 +166,10 @@ attn_exact_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   pdl_launch_dependents();
 
   if (warp == 0) {
-    // ---------------- TMA producer
-    if (lane == 0) {
-      pdl_wait();
+    // ---------------- TMA producer: the whole warp runs the loop, lane 0 issues
+    const bool issuer = lane == 0;
+    pdl_wait();
+    if (issuer) {
       const int n_tiles = t_rows[1] > 0 ? 2 : 1;
       mbar_expect_tx(smem_u32(&q_full), n_tiles * Q_BYTES);
       for (int x = 0; x < n_tiles; ++x)
@@ -174,44 +177,82 @@ attn_exact_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         for (int sub = 0; sub < SUB; ++sub)
           ta_tma_load_2d(q_s + x * Q_BYTES + sub * (TA_BM * 128), &map_q, h * HD + sub * 64, qs + t_m0[x],
                          smem_u32(&q_full));
-      for (int it = 0; it < n_it; ++it) {
-        // the block's first row in its maps, and the columns of K and of V
-        const CUtensorMap *mk = &map_k, *mv = &map_v;
-        int row, col_k = 0, col_v = 0;
-        if (it < e_pool) {
-          mk = &map_pk;
-          mv = &map_pv;
-          row = a.pool_table != nullptr
-                    ? (g * a.pool_pages + a.pool_table[(size_t)slot * a.pool_pps + it]) * KV_PAGE
-                    : (slot * G + g) * a.pool_capacity + it * TA_BN;
-        } else if (it < e_fc || (it >= e_fs && it < e_ring)) {
-          int cb = it - e_pool;                                  // the block of the cache's rows
-          if (it >= e_fs) {
-            cb = rb0 + it - e_fs;
-            if (cb >= n_rb) cb -= n_rb;
-          }
-          row = a.page_table != nullptr ? (g * a.n_pages + a.page_table[(size_t)slot * a.pps + cb]) * KV_PAGE
-                                        : (slot * G + g) * cap + cb * TA_BN;
-        } else {
-          mk = mv = &map_step;
-          col_k = g * HD;
-          col_v = (G + g) * HD;
-          row = qs + (it < e_fs ? (it - e_fc) * TA_BN : step0 + (it - e_ring) * TA_BN);
+    }
+    // the stage of V whose rows no query of this block sees are still to be cleared (-1: none), and how many were
+    int pending = -1, cleared = 0;
+    uint64_t pending_live = 0;
+    auto clear_pending = [&]() {
+      const int s = pending;
+      pending = -1;
+      return ta_clear_foreign_rows<HD>(v_s + s * KV_BYTES, pending_live, smem_u32(&v_landed), cleared++ & 1,
+                                       smem_u32(&v_full[s]), lane, abort_p);
+    };
+    for (int it = 0; it < n_it; ++it) {
+      // the block's first row in its maps, the columns of K and of V, and which of its rows some query of
+      // this block sees: row i of lane i, rows 32 + i beside it
+      const CUtensorMap *mk = &map_k, *mv = &map_v;
+      int row, col_k = 0, col_v = 0;
+      bool seen[2];
+      if (it < e_pool) {
+        mk = &map_pk;
+        mv = &map_pv;
+        row = a.pool_table != nullptr
+                  ? (g * a.pool_pages + a.pool_table[(size_t)slot * a.pool_pps + it]) * KV_PAGE
+                  : (slot * G + g) * a.pool_capacity + it * TA_BN;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) seen[i] = it * TA_BN + 32 * i + lane < n_pooled;
+      } else if (it < e_fc || (it >= e_fs && it < e_ring)) {
+        int cb = it - e_pool;                                    // the block of the cache's rows
+        if (it >= e_fs) {
+          cb = rb0 + it - e_fs;
+          if (cb >= n_rb) cb -= n_rb;
         }
-        const int s = it % XT_STAGES;
-        const uint32_t phase = ((it / XT_STAGES) & 1) ^ 1u;
-        if (!mbar_wait(smem_u32(&k_empty[s]), phase, abort_p)) break;
+        row = a.page_table != nullptr ? (g * a.n_pages + a.page_table[(size_t)slot * a.pps + cb]) * KV_PAGE
+                                      : (slot * G + g) * cap + cb * TA_BN;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int r = cb * TA_BN + 32 * i + lane;
+          seen[i] = it < e_fc ? r < front_cached
+                              : r < cap && past - 1 - last_row + r - (r > last_row ? cap : 0) >= j_lo;
+        }
+      } else {
+        mk = mv = &map_step;
+        col_k = g * HD;
+        col_v = (G + g) * HD;
+        const int t = it < e_fs ? (it - e_fc) * TA_BN : step0 + (it - e_ring) * TA_BN;
+        row = qs + t;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int key = past + t + 32 * i + lane;
+          seen[i] = it < e_fs ? key < n_front : key >= j_lo && key <= last_pos;
+        }
+      }
+      const uint64_t live = (uint64_t)__ballot_sync(0xffffffffu, seen[1]) << 32 | __ballot_sync(0xffffffffu, seen[0]);
+      const int s = it % XT_STAGES;
+      const uint32_t phase = ((it / XT_STAGES) & 1) ^ 1u;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&k_empty[s]), phase, abort_p))) break;
+      if (issuer) {
         mbar_expect_tx(smem_u32(&k_full[s]), KV_BYTES);
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub)
           ta_tma_load_2d(k_s + s * KV_BYTES + sub * (TA_BN * 128), mk, col_k + sub * 64, row, smem_u32(&k_full[s]));
-        if (!mbar_wait(smem_u32(&v_empty[s]), phase, abort_p)) break;
-        mbar_expect_tx(smem_u32(&v_full[s]), KV_BYTES);
+      }
+      // (the stages waited for above and below held block it - 3, whose products need no later block)
+      if (pending >= 0 && !clear_pending()) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&v_empty[s]), phase, abort_p))) break;
+      if (~live) {
+        pending = s;
+        pending_live = live;
+      }
+      if (issuer) {
+        const uint32_t bar = ~live ? smem_u32(&v_landed) : smem_u32(&v_full[s]);
+        mbar_expect_tx(bar, KV_BYTES);
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub)
-          ta_tma_load_2d(v_s + s * KV_BYTES + sub * (TA_BN * 128), mv, col_v + sub * 64, row, smem_u32(&v_full[s]));
+          ta_tma_load_2d(v_s + s * KV_BYTES + sub * (TA_BN * 128), mv, col_v + sub * 64, row, bar);
       }
     }
+    if (pending >= 0) clear_pending();
   } else if (warp == 1 || warp == XT_MMA_B) {
     // ---------------- MMA issuers, one per tile: the whole warp runs the loop, lane 0 issues
     const int x = warp == 1 ? 0 : 1;
@@ -468,8 +509,8 @@ static int launch_exact_tc(const void* q, const void* kv_step, const void* k_cac
 using namespace yalm;
 
 // yalm_attention_exact_prefill for head sizes 64 and 128 (same arguments and meaning, plus the sizes of
-// the caches: n_slots, and n_tokens, and the status word for the bounded waits).  q_start, seq_slot,
-// slot_pos and the page tables are read before the wait on the previous kernel.
+// the caches: n_slots, and n_tokens, and the status word for the bounded waits).  q_start, seq_slot and
+// slot_pos are read before the wait on the previous kernel, the page tables after it.
 extern "C" int yalm_attention_exact_tc(const void* q, const void* kv_step, const void* k_cache, const void* v_cache,
                                        const int* q_start, const int* seq_slot, const int* slot_pos, void* out,
                                        int dtype, int n_tokens, int n_seqs, int max_q_len, int n_slots, int H, int G,

@@ -76,7 +76,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   extern __shared__ uint8_t ta_smem[];
   __shared__ __align__(8) uint64_t q_full, s_full[2][2], p_ready[2][2], pv_done[2][2];
   __shared__ __align__(8) uint64_t k_full[TA_KSTAGES], k_empty[TA_KSTAGES];
-  __shared__ __align__(8) uint64_t v_full[TA_VSTAGES], v_empty[TA_VSTAGES];
+  __shared__ __align__(8) uint64_t v_full[TA_VSTAGES], v_empty[TA_VSTAGES], v_landed;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -164,6 +164,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       mbar_init(smem_u32(&k_full[s]), 1);
       mbar_init(smem_u32(&k_empty[s]), 2);
     }
+    mbar_init(smem_u32(&v_landed), 1);
     for (int s = 0; s < TA_VSTAGES; ++s) {
       mbar_init(smem_u32(&v_full[s]), 1);
       mbar_init(smem_u32(&v_empty[s]), 2);
@@ -187,12 +188,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   pdl_launch_dependents();
 
   if (warp == 0) {
-    // ---------------- TMA producer
-    if (lane == 0) {
+    // ---------------- TMA producer: the whole warp runs the loop, lane 0 issues
+    const bool issuer = lane == 0;
+    if (issuer) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_q)) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_k)) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_v)) : "memory");
-      pdl_wait();
+    }
+    pdl_wait();
+    if (issuer) {
       const int n_tiles = t_rows[1] > 0 ? 2 : 1;
       mbar_expect_tx(smem_u32(&q_full), n_tiles * Q_BYTES);
       for (int x = 0; x < n_tiles; ++x)
@@ -200,26 +204,43 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         for (int sub = 0; sub < SUB; ++sub)
           ta_tma_load_2d(q_s + x * Q_BYTES + sub * (TA_BM * 128), &map_q, h * HD + sub * 64,
                          qs + t_m0[x], smem_u32(&q_full));
-      for (int it = 0; it < n_it; ++it) {
-        // the block's first row in the maps, and the columns of K and of V
-        const int kb = kb_lo + it;
-        int row = qs + kb * TA_BN, col_k = g * HD, col_v = (G + g) * HD;
-        const CUtensorMap *mk = &map_k, *mv = &map_v;
-        if (RING && kb >= n_ring) {
-          row = qs + step0 + (kb - n_ring) * TA_BN;
-          mk = mv = &map_step;
-        } else if (RING || ca.on) {
-          col_k = col_v = 0;
-          int cb = kb;                                        // the block of the cache's rows
-          if constexpr (RING) cb = rb0 + kb - (rb0 + kb >= n_rb ? n_rb : 0);
-          if (ca.page_table != nullptr)
-            row = (g * ca.n_pages + ca.page_table[(size_t)slot * ca.pages_per_slot + cb]) * KV_PAGE;
-          else
-            row = (slot * G + g) * ca.capacity + cb * TA_BN;
+    }
+    // the stage of V whose foreign rows are still to be cleared (-1: none), and how many were
+    int pending = -1, cleared = 0;
+    uint64_t pending_live = 0;
+    auto clear_pending = [&]() {
+      const int s = pending;
+      pending = -1;
+      return ta_clear_foreign_rows<HD>(v_s + s * KV_BYTES, pending_live, smem_u32(&v_landed), cleared++ & 1,
+                                       smem_u32(&v_full[s]), lane, abort_p);
+    };
+    for (int it = 0; it < n_it; ++it) {
+      // the block's first row in the maps, the columns of K and of V, and how many of its rows the
+      // sequence owns
+      const int kb = kb_lo + it;
+      int row = qs + kb * TA_BN, col_k = g * HD, col_v = (G + g) * HD;
+      int own = past + q_len - kb * TA_BN;
+      const CUtensorMap *mk = &map_k, *mv = &map_v;
+      if (RING && kb >= n_ring) {
+        row = qs + step0 + (kb - n_ring) * TA_BN;
+        own = q_len - step0 - (kb - n_ring) * TA_BN;
+        mk = mv = &map_step;
+      } else if (RING || ca.on) {
+        col_k = col_v = 0;
+        int cb = kb;                                          // the block of the cache's rows
+        if constexpr (RING) {
+          cb = rb0 + kb - (rb0 + kb >= n_rb ? n_rb : 0);
+          own = min(ca.capacity, past) - cb * TA_BN;
         }
-        {
-          const int s = it % TA_KSTAGES;
-          if (!mbar_wait(smem_u32(&k_empty[s]), ((it / TA_KSTAGES) & 1) ^ 1u, abort_p)) break;
+        if (ca.page_table != nullptr)
+          row = (g * ca.n_pages + ca.page_table[(size_t)slot * ca.pages_per_slot + cb]) * KV_PAGE;
+        else
+          row = (slot * G + g) * ca.capacity + cb * TA_BN;
+      }
+      {
+        const int s = it % TA_KSTAGES;
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&k_empty[s]), ((it / TA_KSTAGES) & 1) ^ 1u, abort_p))) break;
+        if (issuer) {
           const uint32_t bar = smem_u32(&k_full[s]);
           mbar_expect_tx(bar, KV_BYTES);
 #pragma unroll
@@ -227,10 +248,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             ta_tma_load_2d(k_s + s * KV_BYTES + sub * (TA_BN * 128), mk, col_k + sub * 64,
                            row, bar);
         }
-        {
-          const int s = it % TA_VSTAGES;
-          if (!mbar_wait(smem_u32(&v_empty[s]), ((it / TA_VSTAGES) & 1) ^ 1u, abort_p)) break;
-          const uint32_t bar = smem_u32(&v_full[s]);
+      }
+      // (the stages waited for above and below held block it - 3, whose products need no later block)
+      if (pending >= 0 && !clear_pending()) break;
+      {
+        const int s = it % TA_VSTAGES;
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&v_empty[s]), ((it / TA_VSTAGES) & 1) ^ 1u, abort_p))) break;
+        if (own < TA_BN) {
+          pending = s;
+          pending_live = own > 0 ? (1ull << own) - 1 : 0;
+        }
+        if (issuer) {
+          const uint32_t bar = own < TA_BN ? smem_u32(&v_landed) : smem_u32(&v_full[s]);
           mbar_expect_tx(bar, KV_BYTES);
 #pragma unroll
           for (int sub = 0; sub < SUB; ++sub)
@@ -239,6 +268,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
       }
     }
+    if (pending >= 0) clear_pending();
   } else if (warp == 1 || warp == TA_MMA_B) {
     // ---------------- MMA issuers, one per tile: the whole warp runs the loop, lane 0 issues
     {

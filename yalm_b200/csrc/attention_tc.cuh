@@ -148,6 +148,30 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// V's rows of a key block that lie beyond what the sequence owns (another sequence's rows of the step, rows of
+// the cache or of the pooled rows that this sequence has not written, the next block of rows where a capacity is
+// no multiple of 64) come with a whole-block copy.  Their weights are zero, but zero times an infinity or a NaN
+// is a NaN, so such a block is completed in two steps: its copy arrives on `landed`, and the producer warp clears
+// the rows whose bit in `live` is not set before it completes `full`, which the product waits for.  (A row of
+// 128 bytes keeps its place under the swizzle, which only permutes 16-byte pieces inside it.)  Called by a whole
+// warp; false if a wait gave up.
+template <int HD>
+__device__ __forceinline__ bool ta_clear_foreign_rows(uint32_t v_block, uint64_t live, uint32_t landed, uint32_t parity,
+                                                      uint32_t full, int lane, volatile int* abort_flag) {
+  if (!__all_sync(0xffffffffu, mbar_wait(landed, parity, abort_flag))) return false;
+#pragma unroll
+  for (int sub = 0; sub < HD / 64; ++sub)
+#pragma unroll 4
+    for (int r = lane >> 3; r < TA_BN; r += 4)
+      if (!((live >> r) & 1))
+        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};"
+                     ::"r"(v_block + (uint32_t)(sub * (TA_BN * 128) + r * 128 + (lane & 7) * 16)), "r"(0) : "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) mbar_arrive(full);
+  return true;
+}
+
 typedef CUresult (*TaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
