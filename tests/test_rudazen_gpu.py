@@ -79,10 +79,12 @@ def test_sum_norm(ops, dim, rows, dt):
 @pytest.mark.parametrize("layout", ["halves", "neighbours"])
 @pytest.mark.parametrize("norm", ["row", "head", "none"])
 @pytest.mark.parametrize("H, G, hd, dims, n", [(9, 3, 128, 64, 90), (2, 1, 256, 256, 3), (3, 3, 196, 8, 75),
-                                               (1, 1, 4, 0, 1), (2, 2, 128, 12, 20), (2, 1, 30, 8, 20)])
+                                               (1, 1, 4, 0, 1), (2, 2, 128, 12, 20), (2, 1, 30, 8, 20),
+                                               (32, 8, 256, 0, 3), (394, 1, 30, 8, 2)])
 def test_projection_store_by_heads(ops, layout, norm, H, G, hd, dims, n):
     """The store kernel's two forms (whole 16-byte accesses; other sizes element by element: 12 rotated features
-    in halves, heads of 30) in float64's light: head sizes up to 256, several blocks per token, one slice and three."""
+    in halves, heads of 30) in float64's light: head sizes up to 256, several blocks per token, one slice and three,
+    rows that fill 48 KB of shared memory to the last bytes (12,288 floats; 12,283 of the other form)."""
     g = torch.Generator().manual_seed(H * hd + dims + n)
     row = (H + 2 * G) * hd
     freq = torch.tensor([50.0 ** (-2.0 * i / max(dims, 2)) for i in range(max(dims // 2, 1))])
@@ -112,7 +114,7 @@ def test_projection_store_by_heads(ops, layout, norm, H, G, hd, dims, n):
             x[..., first], x[..., second] = u * c - w * sn, w * c + u * sn
         if norm == "head":
             x = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5)
-        # sums of three slices and a bias, a norm over up to 1,152 features and one rotation in 32 bits: some
+        # sums of three slices and a bias, a norm over up to 11,820 features and one rotation in 32 bits: some
         # ten roundings of values of up to 10
         assert (q_out.cpu().view(n, H, hd) - x[:, :H]).abs().max().item() <= 2e-5
         assert (kv_step[:, 0].cpu() - x[:, H:]).abs().max().item() <= 2e-5

@@ -441,8 +441,9 @@ extern "C" int yalm_qk_norm_rope_store(const float* qkv, int n_partials, long lo
   }
   const uintptr_t bases = (uintptr_t)qkv | (uintptr_t)bias | (uintptr_t)q_norm | (uintptr_t)k_norm | (uintptr_t)q_out |
                           (uintptr_t)kv_step | (uintptr_t)k_cache | (uintptr_t)v_cache;
+  // (a launch without the attribute below has 48 KB of shared memory for the kernel's own variables too)
   const bool vec = hd % 4 == 0 && dims % (neighbours ? 4 : 8) == 0 && (partial_stride & 3) == 0 && (bases & 15) == 0 &&
-                   (size_t)(row + dims) * sizeof(float) <= 48 * 1024;
+                   (size_t)(row + dims) * sizeof(float) <= 48 * 1024 - QKS_WARPS * sizeof(float2);
 #define YALM_QKS(T)                                                                                   \
   do {                                                                                                \
     if (vec) {                                                                                        \
@@ -453,7 +454,7 @@ extern "C" int yalm_qk_norm_rope_store(const float* qkv, int n_partials, long lo
                  (T*)k_cache, (T*)v_cache, H, G, hd, has_v, capacity, write_cache, page_table, pages_per_slot, n_pages); \
       break;                                                                                          \
     }                                                                                                 \
-    static size_t attr = 48 * 1024;                                                                   \
+    static size_t attr = 48 * 1024 - 33 * sizeof(float);                                              \
     if (smem > attr) {                                                                                \
       cudaError_t e = cudaFuncSetAttribute(qk_norm_rope_store_kernel<T>,                              \
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
