@@ -121,12 +121,18 @@ def test_fma_matrix_product_is_true_32_bit(ops, shape):
     assert (out.double() - ah.double() @ w.double().T).abs().max() <= 3e-6 * math.sqrt(K) * ref.abs().max()
 
 
-@pytest.mark.parametrize("shape", [(16, 33, 4), (17, 64, 68), (8, 17, 576), (64, 129, 36), (129, 2049, 20),
-                                   (600, 2048, 132), (700, 640, 33), (148 * 2 + 1, 4100, 64)])
+@pytest.mark.parametrize("tile, shape", [
+    ((32, 64), (16, 33, 4)), ((32, 64), (17, 64, 68)), ((32, 64), (8, 17, 576)), ((32, 64), (64, 129, 36)),
+    ((32, 64), (129, 2049, 20)), ((32, 64), (600, 2048, 132)), ((32, 64), (700, 640, 33)),
+    ((32, 64), (148 * 2 + 1, 4100, 64)), ((128, 128), (1001, 2047, 68)), ((128, 128), (600, 16385, 20)),
+    ((128, 128), (1001, 2050, 35)), ((64, 128), (505, 2300, 36)), ((64, 128), (505, 2303, 21))])
 @pytest.mark.parametrize("store", [torch.float32, torch.bfloat16])
-def test_fma_matrix_product_kernels_give_one_chain(ops, shape, store):
-    """Few rows, every tile shape, remainders in all three sizes: the same bits from each of them."""
+def test_fma_matrix_product_kernels_give_one_chain(ops, tile, shape, store):
+    """Few rows, every tile of 32-bit operands (asserted), the 64 x 64 tile of a 16-bit matrix, remainders in all
+    three sizes, rows of K that 16-byte loads do and do not reach: the same bits from each of them."""
     M, N, K = shape
+    if M > 16:
+        assert ops.gemm_simt_tile(M, N) == tile
     a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV).to(store)
     out = torch.full((M, N), float("nan"), device=DEV)
     ops.gemm_simt(a, w, out)
@@ -138,6 +144,23 @@ def test_fma_matrix_product_kernels_give_one_chain(ops, shape, store):
         few = torch.empty(rows, N, device=DEV)
         ops.gemm_simt(a[M - rows:].contiguous(), w, few)
         assert torch.equal(few, out[M - rows:])
+
+
+@pytest.mark.parametrize("M", [65535 * 32, 65535 * 32 + 1, 65535 * 64])
+def test_fma_matrix_product_of_as_many_rows_as_a_grid_takes(ops, M):
+    """65,535 rows of blocks: beyond 32 rows each, a narrow product takes a taller tile; 64 rows each is the limit."""
+    N, K = 3, 4
+    assert ops.gemm_simt_tile(M, N) == ((32, 64) if M <= 65535 * 32 else (128, 128))
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops.gemm_simt(a, w, out)
+    few = torch.empty(16, N, device=DEV)
+    for r in (0, M // 2, M - 16):
+        ops.gemm_simt(a[r:r + 16].contiguous(), w, few)
+        assert torch.equal(few, out[r:r + 16])
+    assert not torch.isnan(out).any()
+    with pytest.raises(RuntimeError):
+        ops.gemm_simt(torch.empty(65535 * 64 + 1, K, device=DEV), w, torch.empty(65535 * 64 + 1, N, device=DEV))
 
 
 @pytest.mark.parametrize("shape", [(1, 128, 64), (3, 200, 72), (16, 384, 512), (40, 1000, 320),

@@ -120,6 +120,8 @@ int yalm_attention_prefill_tc_ring(const void* q, const void* kv_step, const voi
 
 int yalm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, void* out,
                    int out_dtype, int M, int N, int K, int accumulate, cudaStream_t stream);
+// rows * 1000 + columns of the tile that a product of 32-bit operands with more than 16 rows takes
+int yalm_gemm_simt_tile(int M, int N);
 
 // params: null, or two 64-bit words on the device that replace `seed` and `temperature`
 // (the temperature's float bits in the low half of the second word)

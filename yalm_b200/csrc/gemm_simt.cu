@@ -264,7 +264,8 @@ static int launch_tile(const void* A, const void* W, void* out, int M, int N, in
 
 // The tile shape for an [M, N] product of 32-bit operands, by estimated time.  Measured at K = 2,048, us: a
 // block of 128 x 128 alone on its SM 216, two of them 380; of 64 x 128 140 and 250; 32 x 64 tiles 0.27 each
-// over the whole device, and no less than 66.
+// over the whole device, and no less than 66.  0: 128 x 128, 1: 64 x 128, 2: 32 x 64.
+constexpr long long SIMT_MAX_ROWS = 65535LL * 64;             // (a grid has up to 65,535 rows of blocks)
 static int simt_tile(int M, int N) {
   auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
   auto rounds = [](long long b, double one, double two) {
@@ -273,7 +274,8 @@ static int simt_tile(int M, int N) {
   };
   const double t128 = rounds(blocks(128, 128), 216, 380), t64 = rounds(blocks(64, 128), 140, 250);
   const double small = 0.27 * (double)blocks(32, 64) + 20, t32 = small > 66 ? small : 66;
-  return t128 <= t64 && t128 <= t32 ? 0 : t64 <= t32 ? 1 : 2;
+  const bool can32 = M <= 65535LL * 32;
+  return t128 <= t64 && (t128 <= t32 || !can32) ? 0 : t64 <= t32 || !can32 ? 1 : 2;
 }
 
 template <typename TA, typename TW, typename TO>
@@ -317,6 +319,7 @@ extern "C" int yalm_gemm_simt(const void* A, int a_dtype, const void* W, int w_d
                               cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return -2;
+  if (M > SIMT_MAX_ROWS) return -4;
   if (a_dtype == DT_F32 && w_dtype == DT_F32)
     return launch_simt<float, float>(A, W, out, out_dtype, M, N, K, accumulate, stream);
   if (a_dtype == DT_BF16 && w_dtype == DT_BF16)
@@ -333,4 +336,10 @@ extern "C" int yalm_gemm_simt(const void* A, int a_dtype, const void* W, int w_d
   if (a_dtype == DT_F16 && w_dtype == DT_F32)
     return launch_simt<__half, float>(A, W, out, out_dtype, M, N, K, accumulate, stream);
   return -3;
+}
+
+// The tile that more than FEW_ROWS rows of 32-bit operands run on: its rows times 1,000 plus its columns.
+extern "C" int yalm_gemm_simt_tile(int M, int N) {
+  const int t = simt_tile(M, N);
+  return t == 0 ? 128128 : t == 1 ? 64128 : 32064;
 }

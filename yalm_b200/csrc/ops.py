@@ -73,6 +73,7 @@ _SIGNATURES = {
     "yalm_attention_decode_mma_fused": [_vp, _i, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i,
                                         _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _i, _i, _vp],
     "yalm_gemm_simt": [_vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
+    "yalm_gemm_simt_tile": [_i, _i],
     "yalm_sample": [_vp, _i, _i, _f, _ull, _vp, _vp, _vp, _vp, _vp, _vp],
     "yalm_gemm_tc": [_vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "yalm_gemm_tc_available": [],
@@ -593,6 +594,11 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: b
     _check(lib().yalm_gemm_simt(_p(a), dtype_code(a.dtype), _p(w), dtype_code(w.dtype), _p(out),
                                 dtype_code(out.dtype), M, N, K, 1 if accumulate else 0, _stream()),
            "gemm_simt")
+
+
+def gemm_simt_tile(M: int, N: int) -> tuple:
+    """(rows, columns) of the tile that ``gemm_simt`` takes for 32-bit operands with more than 16 rows."""
+    return divmod(lib().yalm_gemm_simt_tile(int(M), int(N)), 1000)
 
 
 GEMM_STORE, GEMM_ADD, GEMM_SILU_MUL, GEMM_SPLIT, GEMM_SILU_PAIRED = 0, 1, 2, 3, 4
