@@ -300,7 +300,7 @@ def test_tensor_core_attention_with_unrounded_weights(ops, hd, window, pool, dt)
     assert status.item() == 0
 
 
-@pytest.mark.parametrize("H, dk, dv", [(3, 24, 16), (1, 8, 40), (2, 20, 12), (2, 128, 64), (1, 200, 9), (2, 64, 128), (1, 384, 24), (1, 301, 16)])
+@pytest.mark.parametrize("H, dk, dv", [(3, 24, 16), (1, 8, 40), (2, 20, 12), (2, 128, 64), (1, 200, 9), (2, 64, 128), (1, 384, 24), (1, 301, 16), (2, 20, 132)])
 def test_gated_recurrence_in_portions(ops, H, dk, dv):
     g = torch.Generator().manual_seed(dk)
     D = 32
@@ -334,6 +334,30 @@ def test_gated_recurrence_in_portions(ops, H, dk, dv):
         ref = plain_gated_recurrence(w, "r", m, h, 1e-5)
         assert (torch.cat(got[s]) - ref).abs().max().item() <= 3e-5 * max(1.0, ref.abs().max().item()), s
     assert bool((state[1] == 7.0).all())
+
+
+@pytest.mark.parametrize("q_lens", [[0, 2, 1], [1, 0, 2], [3, 0, 0], [0, 0, 3]])
+def test_gated_recurrence_of_uneven_steps(ops, q_lens):
+    """As many tokens as sequences, but not one each: every sequence's bits are those of a step of its own."""
+    H, dk, dv, slots = 2, 20, 68, [2, 0, 3]
+    g = torch.Generator().manual_seed(sum((i + 1) * q for i, q in enumerate(q_lens)))
+    row = 2 * H * dk + H * dv
+    proj, fb, lower = torch.randn(3, row, generator=g), torch.randn(H * dk, generator=g), torch.rand(H * dk, generator=g)
+    s0 = torch.randn(4, H, dk, dv, generator=g)
+
+    def run(rows, lens, which, state):
+        n = rows.shape[0]
+        out, act = torch.full((n, H * dv), float("nan"), device=DEV), torch.empty(n, row, device=DEV)
+        ops.gated_recurrence(rows.to(DEV), 1, fb.to(DEV), lower.to(DEV), B(lens, which), state, out, H, dk, dv, act)
+        return out
+    got_state = s0.to(DEV)
+    got = run(proj, q_lens, slots, got_state)
+    want_state, at = s0.to(DEV), 0
+    for q, s in zip(q_lens, slots):
+        for t in range(at, at + q):
+            assert torch.equal(got[t], run(proj[t:t + 1], [1], [s], want_state)[0])
+        at += q
+    assert torch.equal(got_state, want_state)
 
 
 # ------------------------------------------------------------------ the engine against the plain model

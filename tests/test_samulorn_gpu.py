@@ -181,6 +181,31 @@ def test_delta_rule_one_token(ops, H, G, dk, dv):
         assert close(step, scan.cpu(), 1e-5)
 
 
+@pytest.mark.parametrize("q_lens", [[0, 2, 1], [1, 0, 2], [3, 0, 0], [0, 0, 3]])
+def test_delta_rule_of_uneven_steps(ops, q_lens):
+    """As many tokens as sequences, but not one each: every sequence's bits are those of steps of its own."""
+    H, G, dk, dv, slots = 2, 1, 60, 68, [2, 0, 3]
+    g = torch.Generator().manual_seed(sum((i + 1) * q for i, q in enumerate(q_lens)))
+    act = torch.randn(3, ops.delta_row(H, G, dk, dv), generator=g)
+    act[:, :2 * G * dk] *= dk ** -0.5
+    z, dt, a_log = torch.randn(3, H * dk + H * dv, generator=g), torch.randn(H * dk, generator=g), torch.zeros(H)
+    s0 = torch.randn(4, H, dk, dv, generator=g)
+
+    def run(lo, hi, lens, which, state):
+        gate, out = torch.empty(hi - lo, H * dv, device=DEV), torch.full((hi - lo, H * dv), float("nan"), device=DEV)
+        ops.delta_scan(act[lo:hi].to(DEV), z[lo:hi].to(DEV), 1, dt.to(DEV), a_log.to(DEV), gate, B(lens, which), state, out,
+                       H, G, dk, dv)
+        return out
+    got_state = s0.to(DEV)
+    got = run(0, 3, q_lens, slots, got_state)
+    want_state, at = s0.to(DEV), 0
+    for q, s in zip(q_lens, slots):
+        for t in range(at, at + q):
+            assert torch.equal(got[t], run(t, t + 1, [1], [s], want_state)[0])
+        at += q
+    assert torch.equal(got_state, want_state)
+
+
 @pytest.mark.parametrize("W, blocks", [(48, 3), (64, 1), (30, 5), (512, 4)])
 def test_rglru_kernels(ops, W, blocks):
     g = torch.Generator().manual_seed(W)

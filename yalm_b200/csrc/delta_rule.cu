@@ -462,11 +462,10 @@ delta_step_kernel(const float* __restrict__ act, int row, const int* __restrict_
   const int b = blockIdx.z, h = blockIdx.y, hq = h / (H / G), hp = (H + 3) & ~3;
   const int cq = threadIdx.x % CQ, rg = threadIdx.x / CQ;
   const int c0 = blockIdx.x * 4 * CQ, col = c0 + cq * 4;
-  const int slot = seq_slot[b], t = q_start[b];
+  const int slot = seq_slot[b], t0 = q_start[b], t1 = q_start[b + 1];
   const bool on = col < dv;
   float* st = state + ((size_t)slot * H + h) * dk * dv + col;
   pdl_wait();
-  const float* src = act + (size_t)t * row;
   float4 S[ROWS];
 #pragma unroll
   for (int j = 0; j < ROWS; ++j) {
@@ -474,51 +473,55 @@ delta_step_kernel(const float* __restrict__ act, int row, const int* __restrict_
     S[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (on && r < dk) S[j] = *reinterpret_cast<const float4*>(st + (size_t)r * dv);
   }
-  for (int i = threadIdx.x; i < RG * ROWS; i += 256) {
-    qs[i] = i < dk ? src[hq * dk + i] : 0.f;
-    ks[i] = i < dk ? src[G * dk + hq * dk + i] : 0.f;
-    gs[i] = i < dk ? src[2 * G * dk + H * dv + hp + h * dk + i] : 0.f;
-  }
-  __syncthreads();
-  float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+  // one token; none or several where a caller's step has as many tokens as sequences but does not deal them out evenly
+  for (int t = t0; t < t1; ++t) {
+    const float* src = act + (size_t)t * row;
+    for (int i = threadIdx.x; i < RG * ROWS; i += 256) {
+      qs[i] = i < dk ? src[hq * dk + i] : 0.f;
+      ks[i] = i < dk ? src[G * dk + hq * dk + i] : 0.f;
+      gs[i] = i < dk ? src[2 * G * dk + H * dv + hp + h * dk + i] : 0.f;
+    }
+    __syncthreads();
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int j = 0; j < ROWS; ++j) {
-    const float g = gs[rg + j * RG], k = ks[rg + j * RG];
-    S[j].x = fmaf(g, S[j].x, S[j].x); S[j].y = fmaf(g, S[j].y, S[j].y);
-    S[j].z = fmaf(g, S[j].z, S[j].z); S[j].w = fmaf(g, S[j].w, S[j].w);
-    d.x = fmaf(k, S[j].x, d.x); d.y = fmaf(k, S[j].y, d.y);
-    d.z = fmaf(k, S[j].z, d.z); d.w = fmaf(k, S[j].w, d.w);
-  }
-  *reinterpret_cast<float4*>(&part[rg][4 * cq]) = d;
-  __syncthreads();
-  if (threadIdx.x < 4 * CQ) {
-    const int c = c0 + threadIdx.x;
-    float sum = 0.f;
+    for (int j = 0; j < ROWS; ++j) {
+      const float g = gs[rg + j * RG], k = ks[rg + j * RG];
+      S[j].x = fmaf(g, S[j].x, S[j].x); S[j].y = fmaf(g, S[j].y, S[j].y);
+      S[j].z = fmaf(g, S[j].z, S[j].z); S[j].w = fmaf(g, S[j].w, S[j].w);
+      d.x = fmaf(k, S[j].x, d.x); d.y = fmaf(k, S[j].y, d.y);
+      d.z = fmaf(k, S[j].z, d.z); d.w = fmaf(k, S[j].w, d.w);
+    }
+    *reinterpret_cast<float4*>(&part[rg][4 * cq]) = d;
+    __syncthreads();
+    if (threadIdx.x < 4 * CQ) {
+      const int c = c0 + threadIdx.x;
+      float sum = 0.f;
 #pragma unroll
-    for (int g = 0; g < RG; ++g) sum += part[g][threadIdx.x];
-    u_s[threadIdx.x] = c < dv ? src[2 * G * dk + H * dv + h] * (src[2 * G * dk + h * dv + c] - sum) : 0.f;
-  }
-  __syncthreads();
-  const float4 u = *reinterpret_cast<const float4*>(&u_s[4 * cq]);
-  d = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int g = 0; g < RG; ++g) sum += part[g][threadIdx.x];
+      u_s[threadIdx.x] = c < dv ? src[2 * G * dk + H * dv + h] * (src[2 * G * dk + h * dv + c] - sum) : 0.f;
+    }
+    __syncthreads();
+    const float4 u = *reinterpret_cast<const float4*>(&u_s[4 * cq]);
+    d = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int j = 0; j < ROWS; ++j) {
-    const int r = rg + j * RG;
-    const float k = ks[r], q = qs[r];
-    S[j].x = fmaf(k, u.x, S[j].x); S[j].y = fmaf(k, u.y, S[j].y);
-    S[j].z = fmaf(k, u.z, S[j].z); S[j].w = fmaf(k, u.w, S[j].w);
-    d.x = fmaf(S[j].x, q, d.x); d.y = fmaf(S[j].y, q, d.y);
-    d.z = fmaf(S[j].z, q, d.z); d.w = fmaf(S[j].w, q, d.w);
-    if (on && r < dk) *reinterpret_cast<float4*>(st + (size_t)r * dv) = S[j];
-  }
-  *reinterpret_cast<float4*>(&part[rg][4 * cq]) = d;
-  __syncthreads();
-  if (threadIdx.x < 4 * CQ) {
-    const int c = c0 + threadIdx.x;
-    float sum = 0.f;
+    for (int j = 0; j < ROWS; ++j) {
+      const int r = rg + j * RG;
+      const float k = ks[r], q = qs[r];
+      S[j].x = fmaf(k, u.x, S[j].x); S[j].y = fmaf(k, u.y, S[j].y);
+      S[j].z = fmaf(k, u.z, S[j].z); S[j].w = fmaf(k, u.w, S[j].w);
+      d.x = fmaf(S[j].x, q, d.x); d.y = fmaf(S[j].y, q, d.y);
+      d.z = fmaf(S[j].z, q, d.z); d.w = fmaf(S[j].w, q, d.w);
+      if (on && r < dk) *reinterpret_cast<float4*>(st + (size_t)r * dv) = S[j];
+    }
+    *reinterpret_cast<float4*>(&part[rg][4 * cq]) = d;
+    __syncthreads();
+    if (threadIdx.x < 4 * CQ) {
+      const int c = c0 + threadIdx.x;
+      float sum = 0.f;
 #pragma unroll
-    for (int g = 0; g < RG; ++g) sum += part[g][threadIdx.x];
-    if (c < dv) out[((size_t)t * H + h) * dv + c] = sum;
+      for (int g = 0; g < RG; ++g) sum += part[g][threadIdx.x];
+      if (c < dv) out[((size_t)t * H + h) * dv + c] = sum;
+    }
   }
 }
 
@@ -571,7 +574,7 @@ extern "C" int yalm_delta_scan(float* act, const float* z, int n_partials, long 
              partial_stride, dt_bias, a_log, gate, H, dk, dv);
   YALM_LAUNCH_CHECK();
   const bool vec = dk % 4 == 0 && dv % 4 == 0 && (((uintptr_t)act) & 15) == 0;
-  // one token per sequence (a step has no sequence without tokens), whole 16-byte accesses
+  // one token per sequence, whole 16-byte accesses
   if (n_tokens == n_seqs && dk <= 128 && vec && (((uintptr_t)state) & 15) == 0) {
 #define YALM_DSTEP(R, CQ)                                                                                    \
   launch_pdl(delta_step_kernel<R, CQ>, dim3((dv + 4 * CQ - 1) / (4 * CQ), H, n_seqs), dim3(256), 0, stream,  \

@@ -614,65 +614,68 @@ state_step_kernel(const float* __restrict__ act, const float* __restrict__ bonus
   const int b = blockIdx.z, h = blockIdx.y;
   const int cq = threadIdx.x % CQ, rg = threadIdx.x / CQ;
   const int col = (blockIdx.x * CQ + cq) * 4;
-  const int slot = seq_slot[b], t = q_start[b];
+  const int slot = seq_slot[b], t0 = q_start[b], t1 = q_start[b + 1];
   const int row = (WKV ? 3 : 2) * H * dk + H * dv;
   float* st = state + ((size_t)slot * H + h) * dk * dv + col;
   const bool on = col < dv;
   pdl_wait();
-  const float* src = act + (size_t)t * row;
-  for (int i = threadIdx.x; i < dk; i += 256) {
+  // one token; none or several where a caller's step has as many tokens as sequences but does not deal them out evenly
+  for (int t = t0; t < t1; ++t) {
+    const float* src = act + (size_t)t * row;
+    for (int i = threadIdx.x; i < dk; i += 256) {
 #pragma unroll
-    for (int k = 0; k < (WKV ? 3 : 2); ++k) step_s[k * dk + i] = src[k * H * dk + h * dk + i];
-    if constexpr (WKV) step_s[3 * dk + i] = bonus[h * dk + i];
-  }
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f), o = v;
-  if (on) v = *reinterpret_cast<const float4*>(src + (WKV ? 3 : 2) * H * dk + h * dv + col);
-  __syncthreads();
-  if (on) {
-    auto cell = [&](float s, float vj, float q, float f, float k, float u, float& oj) {
-      if constexpr (WKV) {
-        const float kv = k * vj;
-        oj = fmaf(q, fmaf(u, kv, s), oj);
-        return fmaf(f, s, kv);
-      } else {
-        s = fmaf(f, s, (1.0f - f) * vj);
-        oj = fmaf(s, q, oj);
-        return s;
-      }
-    };
-    for (int r0 = rg; r0 < dk; r0 += 4 * RG) {
-      float4 s[4];
+      for (int k = 0; k < (WKV ? 3 : 2); ++k) step_s[k * dk + i] = src[k * H * dk + h * dk + i];
+      if constexpr (WKV) step_s[3 * dk + i] = bonus[h * dk + i];
+    }
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f), o = v;
+    if (on) v = *reinterpret_cast<const float4*>(src + (WKV ? 3 : 2) * H * dk + h * dv + col);
+    __syncthreads();
+    if (on) {
+      auto cell = [&](float s, float vj, float q, float f, float k, float u, float& oj) {
+        if constexpr (WKV) {
+          const float kv = k * vj;
+          oj = fmaf(q, fmaf(u, kv, s), oj);
+          return fmaf(f, s, kv);
+        } else {
+          s = fmaf(f, s, (1.0f - f) * vj);
+          oj = fmaf(s, q, oj);
+          return s;
+        }
+      };
+      for (int r0 = rg; r0 < dk; r0 += 4 * RG) {
+        float4 s[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (r0 + j * RG < dk) s[j] = *reinterpret_cast<const float4*>(st + (size_t)(r0 + j * RG) * dv);
+        for (int j = 0; j < 4; ++j)
+          if (r0 + j * RG < dk) s[j] = *reinterpret_cast<const float4*>(st + (size_t)(r0 + j * RG) * dv);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = r0 + j * RG;
-        if (r >= dk) break;
-        const float q = step_s[r], f = step_s[dk + r];
-        const float k = WKV ? step_s[(N_VEC - 2) * dk + r] : 0.f, u = WKV ? step_s[(N_VEC - 1) * dk + r] : 0.f;
-        s[j].x = cell(s[j].x, v.x, q, f, k, u, o.x);
-        s[j].y = cell(s[j].y, v.y, q, f, k, u, o.y);
-        s[j].z = cell(s[j].z, v.z, q, f, k, u, o.z);
-        s[j].w = cell(s[j].w, v.w, q, f, k, u, o.w);
-        *reinterpret_cast<float4*>(st + (size_t)r * dv) = s[j];
+        for (int j = 0; j < 4; ++j) {
+          const int r = r0 + j * RG;
+          if (r >= dk) break;
+          const float q = step_s[r], f = step_s[dk + r];
+          const float k = WKV ? step_s[(N_VEC - 2) * dk + r] : 0.f, u = WKV ? step_s[(N_VEC - 1) * dk + r] : 0.f;
+          s[j].x = cell(s[j].x, v.x, q, f, k, u, o.x);
+          s[j].y = cell(s[j].y, v.y, q, f, k, u, o.y);
+          s[j].z = cell(s[j].z, v.z, q, f, k, u, o.z);
+          s[j].w = cell(s[j].w, v.w, q, f, k, u, o.w);
+          *reinterpret_cast<float4*>(st + (size_t)r * dv) = s[j];
+        }
       }
     }
-  }
-  *reinterpret_cast<float4*>(&part[rg][4 * cq]) = o;
-  __syncthreads();
-  if (threadIdx.x < 4 * CQ) {
-    const int c = blockIdx.x * 4 * CQ + threadIdx.x;
-    float sum = 0.f;
+    *reinterpret_cast<float4*>(&part[rg][4 * cq]) = o;
+    __syncthreads();
+    if (threadIdx.x < 4 * CQ) {
+      const int c = blockIdx.x * 4 * CQ + threadIdx.x;
+      float sum = 0.f;
 #pragma unroll
-    for (int g = 0; g < RG; ++g) sum += part[g][threadIdx.x];
-    if (c < dv) out[((size_t)t * H + h) * dv + c] = sum;
+      for (int g = 0; g < RG; ++g) sum += part[g][threadIdx.x];
+      if (c < dv) out[((size_t)t * H + h) * dv + c] = sum;
+    }
   }
 }
 template <bool WKV>
 static bool launch_state_step(const float* act, const float* bonus, const int* q_start, const int* seq_slot, float* state,
                               float* out, int n_tokens, int n_seqs, int H, int dk, int dv, cudaStream_t stream) {
-  // one token per sequence (a step has no sequence without tokens), whole 16-byte accesses
+  // one token per sequence, whole 16-byte accesses
   if (n_tokens != n_seqs || dv % 4 || dk % 4 || ((((uintptr_t)act) | ((uintptr_t)state)) & 15)) return false;
   const size_t smem = (size_t)(WKV ? 4 : 2) * dk * sizeof(float);
   if (dv <= 64)
