@@ -450,7 +450,7 @@ delta_scan8_kernel(const float* __restrict__ act, int row, const int* __restrict
 // sequences of 16 heads of 128 x 128, 134 MB of state in and out: a whole decode step of two Samulorn layers
 // 417 us with the scan, 352 with this.)
 template <int ROWS, int CQ>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, ROWS == 16 ? 2 : ROWS == 8 ? 3 : 5)
 delta_step_kernel(const float* __restrict__ act, int row, const int* __restrict__ q_start,
                   const int* __restrict__ seq_slot, float* __restrict__ state, float* __restrict__ out, int H, int G,
                   int dk, int dv) {
@@ -474,6 +474,7 @@ delta_step_kernel(const float* __restrict__ act, int row, const int* __restrict_
     if (on && r < dk) S[j] = *reinterpret_cast<const float4*>(st + (size_t)r * dv);
   }
   // one token; none or several where a caller's step has as many tokens as sequences but does not deal them out evenly
+#pragma unroll 1
   for (int t = t0; t < t1; ++t) {
     const float* src = act + (size_t)t * row;
     for (int i = threadIdx.x; i < RG * ROWS; i += 256) {

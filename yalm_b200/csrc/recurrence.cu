@@ -603,7 +603,7 @@ wkv_scan_kernel(const float* __restrict__ act, const float* __restrict__ bonus,
 // above lets every lane pick 8 bytes of its own rows: 64 sequences of 32 heads of 64 x 64, 67 MB of
 // state in and out, 90 us; here 13.)
 template <bool WKV, int CQ>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 state_step_kernel(const float* __restrict__ act, const float* __restrict__ bonus, const int* __restrict__ q_start,
                   const int* __restrict__ seq_slot, float* __restrict__ state, float* __restrict__ out, int H, int dk,
                   int dv) {
@@ -620,6 +620,7 @@ state_step_kernel(const float* __restrict__ act, const float* __restrict__ bonus
   const bool on = col < dv;
   pdl_wait();
   // one token; none or several where a caller's step has as many tokens as sequences but does not deal them out evenly
+#pragma unroll 1
   for (int t = t0; t < t1; ++t) {
     const float* src = act + (size_t)t * row;
     for (int i = threadIdx.x; i < dk; i += 256) {
