@@ -336,6 +336,30 @@ def test_gated_recurrence_in_portions(ops, H, dk, dv):
     assert bool((state[1] == 7.0).all())
 
 
+@pytest.mark.parametrize("H, dk, dv, n", [(2, 128, 128, 3), (16, 64, 132, 30), (3, 20, 64, 2), (40, 36, 60, 2)])
+def test_gated_recurrence_decode_steps_without_a_wait(ops, H, dk, dv, n):
+    """Twenty one-token steps in a row with nothing waited for, in blocks of 32, 64 and 128 value columns, against the
+    same steps in 64 bits (a step adds one rounding of a state that the decays keep bounded, and sums dk terms)."""
+    g = torch.Generator().manual_seed(H * dk + dv)
+    row, slots = 2 * H * dk + H * dv, list(range(n))[::-1]
+    projs = torch.randn(20, n, row, generator=g)
+    fb, lower = torch.randn(H * dk, generator=g), 0.9 * torch.rand(H * dk, generator=g)
+    state = torch.randn(n + 1, H, dk, dv, generator=g)
+    S = state.double()[slots]
+    dev, act, outs = projs.to(DEV), torch.empty(n, row, device=DEV), torch.zeros(20, n, H * dv, device=DEV)
+    state, fbd, ld, b = state.to(DEV), fb.to(DEV), lower.to(DEV), B([1] * n, slots)
+    for p, out in zip(dev, outs):
+        ops.gated_recurrence(p, 1, fbd, ld, b, state, out, H, dk, dv, act)
+    for p, out in zip(projs.double(), outs.cpu()):
+        z = p[:, :H * dk]
+        q, v = (z * torch.sigmoid(z)).view(n, H, dk), p[:, 2 * H * dk:].view(n, H, dv)
+        f = (lower.double() + (1 - lower.double()) * torch.sigmoid(p[:, H * dk:2 * H * dk] + fb.double())).view(n, H, dk)
+        S = f[..., None] * S + (1 - f)[..., None] * v[:, :, None]
+        ref = torch.einsum("nhk,nhkv->nhv", q, S).reshape(n, H * dv)
+        assert (out.double() - ref).abs().max().item() <= 1e-5 * max(1.0, ref.abs().max().item())
+    assert (state[slots].double().cpu() - S).abs().max().item() <= 1e-5
+
+
 @pytest.mark.parametrize("q_lens", [[0, 2, 1], [1, 0, 2], [3, 0, 0], [0, 0, 3]])
 def test_gated_recurrence_of_uneven_steps(ops, q_lens):
     """As many tokens as sequences, but not one each: every sequence's bits are those of a step of its own."""

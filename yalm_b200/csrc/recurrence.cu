@@ -679,12 +679,18 @@ static bool launch_state_step(const float* act, const float* bonus, const int* q
   // one token per sequence, whole 16-byte accesses
   if (n_tokens != n_seqs || dv % 4 || dk % 4 || ((((uintptr_t)act) | ((uintptr_t)state)) & 15)) return false;
   const size_t smem = (size_t)(WKV ? 4 : 2) * dk * sizeof(float);
-  if (dv <= 64)
-    launch_pdl(state_step_kernel<WKV, 16>, dim3(1, H, n_seqs), dim3(256), smem, stream, act, bonus, q_start, seq_slot,
-               state, out, H, dk, dv);
-  else
-    launch_pdl(state_step_kernel<WKV, 32>, dim3((dv + 127) / 128, H, n_seqs), dim3(256), smem, stream, act, bonus, q_start,
-               seq_slot, state, out, H, dk, dv);
+  // wide blocks (rows of 256 or 512 bytes) where they reach half of the SMs, else blocks of 32 columns: a
+  // few sequences' steps are bound by how much of the state is in flight (a Rudazen decode step of one sequence, 16
+  // heads of 128 x 128: 154.8 us in wide blocks, 152.9 with the scan, 152.0 in narrow ones)
+  const int wide = dv <= 64 ? 16 : 32;
+  const bool narrow = (long long)((dv + 4 * wide - 1) / (4 * wide)) * H * n_seqs < 74;
+#define YALM_STEP(CQ)                                                                                             \
+  launch_pdl(state_step_kernel<WKV, CQ>, dim3((dv + 4 * CQ - 1) / (4 * CQ), H, n_seqs), dim3(256), smem, stream, \
+             act, bonus, q_start, seq_slot, state, out, H, dk, dv)
+  if (narrow) YALM_STEP(8);
+  else if (wide == 16) YALM_STEP(16);
+  else YALM_STEP(32);
+#undef YALM_STEP
   return true;
 }
 
