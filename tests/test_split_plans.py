@@ -2,6 +2,8 @@
 block shape (host arithmetic only)."""
 import random
 
+import pytest
+
 from yalm_b200.parts import decode_plan
 from yalm_b200.parts.linear import _valid_splits, plan_splits, plan_splits_many
 
@@ -116,3 +118,28 @@ def test_chunks_per_block_of_the_decode_attention():
     att.rt.decode_attention_warps, att.rt.decode_attention_chunks = 2, 5
     assert att.decode_warps(_Lengths([700] * 16, 1024), 1024, 16) == 2
     assert plan([959], 1024) == 5
+
+
+# (H, hd, positions before the step, window, sequences, tokens of each, us on 64-row tiles, us on 256-row blocks)
+MEASURED_SHORT = [
+    (16, 128, 0, 0, 1, 2, 5.8, 5.5), (16, 128, 0, 0, 16, 2, 7.3, 13.0), (16, 128, 0, 0, 16, 64, 11.5, 13.3),
+    (16, 128, 0, 0, 16, 128, 31.6, 19.0), (16, 128, 1000, 0, 16, 2, 116.1, 73.2), (16, 128, 8000, 0, 16, 64, 945.9, 443.4),
+    (16, 128, 8000, 1024, 16, 16, 128.1, 85.4), (32, 64, 0, 0, 1, 8, 4.6, 5.2), (32, 64, 0, 0, 1, 64, 6.4, 5.3),
+    (32, 64, 0, 0, 4, 2, 5.8, 6.2), (32, 64, 0, 0, 4, 128, 14.8, 8.8), (32, 64, 0, 0, 16, 2, 7.2, 23.2),
+    (32, 64, 0, 0, 16, 128, 26.3, 32.8), (32, 64, 1000, 0, 4, 2, 78.5, 35.3), (32, 64, 1000, 0, 16, 2, 95.0, 137.6),
+    (32, 64, 1000, 0, 16, 128, 217.4, 147.5), (32, 64, 8000, 0, 16, 64, 768.7, 832.7), (32, 64, 8000, 0, 16, 128, 1531.0, 842.3),
+    (32, 64, 8000, 1024, 16, 2, 100.1, 161.0), (32, 64, 5000, 4096, 16, 64, 399.9, 481.9), (32, 64, 5000, 4096, 4, 512, 792.5, 317.2)]
+
+
+@pytest.mark.parametrize("H, hd, past, window, S, q, tiles_us, blocks_us", MEASURED_SHORT)
+def test_short_steps_take_the_attention_kernel_that_measured_faster(H, hd, past, window, S, q, tiles_us, blocks_us):
+    from yalm_b200.parts.attention import short_tiles_win
+    assert short_tiles_win(148, S * q, S, S * past, H, hd, window or None) == (tiles_us < blocks_us)
+
+
+def test_short_steps_count_pooled_and_kept_rows():
+    from yalm_b200.parts.attention import short_tiles_win
+    # 16 heads of 128 behind a window of 64: the 64-row tiles win until enough pooled rows or kept positions are added
+    step = (148, 32, 16, 16 * 100000, 16, 128, 64)
+    assert short_tiles_win(*step)
+    assert not short_tiles_win(*step, pool=64) and not short_tiles_win(*step, keep_first=2000)

@@ -494,9 +494,13 @@ static int launch_exact_tc(const void* q, const void* kv_step, const void* k_cac
   if (rc) return rc;
   // two query tiles, the K and V rings, slack to align to 1024
   const size_t smem = (size_t)2 * TA_BM * HD * 2 + (size_t)2 * XT_STAGES * TA_BN * HD * 2 + 1024;
-  const cudaError_t e =
-      cudaFuncSetAttribute(attn_exact_tc_kernel<HD, T16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
+  static bool attr_set = false;
+  if (!attr_set) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(attn_exact_tc_kernel<HD, T16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
   const dim3 grid(a.H, n_seqs, (max_q_len + 2 * TA_BM - 1) / (2 * TA_BM));
   launch_pdl(attn_exact_tc_kernel<HD, T16>, grid, dim3(XT_THREADS), smem, stream, mq, mk, mv, ms, mpk, mpv, a,
              (T16*)out);

@@ -506,7 +506,7 @@ def attention_prefill_tc_ring(q: torch.Tensor, kv_step: torch.Tensor, k_cache: t
     n_slots = slot_pos.numel() if pt is not None else k_cache.shape[0]
     if pt is None:
         _need(tuple(k_cache.shape[1:]) == (G, capacity, hd),
-              f"attention_prefill_tc_ring: a cache of one block per sequence is [slots, {G}, {capacity}, {hd}]")
+              "attention_prefill_tc_ring: a cache of one block per sequence is [slots, G, capacity, hd]")
     _check(lib().yalm_attention_prefill_tc_ring(_p(q), _p(kv_step), _p(k_cache), _p(v_cache), _p(batch.q_start),
                                                 _p(batch.seq_slot), _p(slot_pos), _p(out),
                                                 dtype_code(q.dtype), q.shape[0], batch.n_seqs,
@@ -836,7 +836,7 @@ def attention_exact_tc(q: torch.Tensor, kv_step: torch.Tensor, k_cache: torch.Te
     n_slots = slot_pos.numel() if pt is not None else k_cache.shape[0]
     if pt is None:
         _need(tuple(k_cache.shape[1:]) == (G, capacity, hd),
-              f"attention_exact_tc: a cache of one block per sequence is [slots, {G}, {capacity}, {hd}]")
+              "attention_exact_tc: a cache of one block per sequence is [slots, G, capacity, hd]")
     pk = pv = ppt = None
     pool = pcap = ppps = pnpg = 0
     if pooled is not None:

@@ -61,6 +61,30 @@ from . import decode_plan, linear
 from .linear import matmul_partials
 
 
+def short_tiles_win(sm_count, n_tokens, n_seqs, past, H, hd, window=None, pool=None, keep_first=None) -> bool:
+    """Whether a step of few tokens for each of many sequences (``past``: their positions before the step, summed)
+    is faster on the 64-row tiles of the mma.sync kernel than on the 256-row blocks of the tcgen05 one, of which an
+    SM holds one, against two (head size 128) or four (64).  By the mean sequence; us per block and per key
+    block of 64 as measured.  Sixteen sequences of 2 tokens, 32 heads of 64: 7 us against 23 without cached keys, 95
+    against 138 on 1,000, 723 against 831 on 8,000; 16 heads of 128: 7 against 13 without, but 116 against 73 on
+    1,000.  Beyond 128 tokens, and where the blocks of all heads and sequences fit the device at once, tcgen05 wins
+    (16 heads of 128, one sequence of 2 tokens: 5.5 us against 5.8, on 8,000 keys 220 against 674)."""
+    if hd not in (64, 128) or n_tokens > 128 * n_seqs:
+        return False
+    if n_seqs * H <= sm_count:         # one key block of a small head: 4.6-5.8 us against 5.2-6.2 up to 16 tokens
+        return hd == 64 and n_tokens <= 16 * n_seqs and n_tokens + past <= 64 * n_seqs
+    length = (n_tokens + past) / n_seqs
+    visible = min(length, window + n_tokens / n_seqs) if window else length
+    if pool:
+        visible += max(0.0, length - window) / pool
+    if keep_first:
+        visible = min(length, visible + keep_first)
+    keys = max(1.0, visible / 64)
+    tiles = n_seqs * H * -(-n_tokens // (64 * n_seqs))
+    resident, per_key_block = (4 * sm_count, 5.7) if hd == 64 else (2 * sm_count, 7.2)
+    return -(-tiles // resident) * (2.0 + per_key_block * keys) < -(-n_seqs * H // sm_count) * (4.3 + 1.7 * keys)
+
+
 def exact_attention(rt, q, kv_step, k_cache, v_cache, batch, slot_pos, o, H, G, hd, capacity, window, pages,
                     scale, chunk=None, pooled=None, pool=None, keep_first=None) -> None:
     """Attention with 32-bit scores, softmax weights and weighted sum: a prompt (or a portion of
@@ -68,7 +92,8 @@ def exact_attention(rt, q, kv_step, k_cache, v_cache, batch, slot_pos, o, H, G, 
     them takes the shape (tcgen05: head sizes 64 and 128; mma.sync: others, and on request); else the FMA kernel, a decode step's few queries split over their keys
     so that the grid fills the device."""
     n = batch.n_tokens
-    if not batch.is_decode and rt.attention in ("auto", "tcgen05") and ops.exact_tc_usable(rt.dtype, hd, chunk):
+    if (not batch.is_decode and rt.attention in ("auto", "tcgen05") and ops.exact_tc_usable(rt.dtype, hd, chunk)
+            and not short_tiles_win(rt.sm_count, n, batch.n_seqs, sum(batch.past), H, hd, window, pool, keep_first)):
         ops.attention_exact_tc(q, kv_step, k_cache, v_cache, batch, slot_pos, o, H, G, hd, capacity, window,
                                rt.status, pages=pages, scale=scale, pooled=pooled, keep_first=keep_first)
         return
