@@ -294,6 +294,7 @@ def _rope_attend(ops, dt, H, G, hd, cap, window, q_lens, slots, n_slots, steps, 
     (16, 1, 64, 24, 24),       # one kv head, a ring of 24 rows shorter than the prompt
     (4, 4, 256, 96, 50),       # the largest head, window inside a larger ring
     (6, 3, 112, 40, 40),
+    (9, 3, 24, 64, 30),        # four lanes per key
 ])
 def test_rotary_cache_write_and_attention(ops, dt, tol, H, G, hd, cap, window):
     err = _rope_attend(ops, dt, H, G, hd, cap, window, q_lens=[33, 1, 60], slots=[4, 0, 2],
@@ -1072,3 +1073,38 @@ def test_tcgen05_attention_keeps_foreign_rows_out(ops, kind, hd, window, cap, po
             outs[-1] += [out[qs[i]:qs[i + 1]].clone() for i in (0, 2)]
     for i, (clean, got) in enumerate(zip(*outs)):
         assert torch.equal(clean, got), (i, int((clean != got).any(-1).nonzero()[0]))
+
+
+@pytest.mark.parametrize("kind", ["step", "ring", "exact"])
+def test_prompt_attention_passes_follow_one_another_without_a_wait(ops, kind):
+    """Several steps of three sequences behind a window, each launched 15 times in a row with the late ring write and
+    the positions' advance between the steps and nothing waited for: the bits of launches that are waited for."""
+    H, G, hd, cap, window, n_slots = 4, 2, 128, 130, 130, 4
+    steps = ([300, 1, 70], [65, 130, 256], [2, 64, 31], [257, 3, 128])
+    outs = []
+    for wait in (True, False):
+        g = torch.Generator().manual_seed(17)
+        kc = torch.zeros(n_slots, G, cap, hd, device=DEV, dtype=torch.bfloat16)
+        vc = torch.zeros_like(kc)
+        slot_pos, status = torch.zeros(n_slots, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ins = [(B(l, [2, 0, 3]), torch.randn(sum(l), H * hd, generator=g).bfloat16().to(DEV),
+                torch.randn(sum(l), 2, G, hd, generator=g).bfloat16().to(DEV)) for l in steps]
+        res = [[torch.zeros_like(q) for _ in range(15)] for _, q, _ in ins]
+        torch.cuda.synchronize()
+        for (b, q, kv), outs_of in zip(ins, res):
+            for o in outs_of:
+                if kind == "step":
+                    ops.attention_prefill_tc(q, kv, b, o, H, G, hd, window, status)
+                elif kind == "ring":
+                    ops.attention_prefill_tc_ring(q, kv, kc, vc, b, slot_pos, o, H, G, hd, cap, window, status)
+                else:
+                    ops.attention_exact_tc(q, kv, kc, vc, b, slot_pos, o, H, G, hd, cap, window, status)
+                if wait:
+                    torch.cuda.synchronize()
+            ops.cache_write(kv, b, kc, vc, slot_pos, G, hd, cap)
+            ops.advance(b, slot_pos)
+        torch.cuda.synchronize()
+        assert status.item() == 0
+        outs.append(res)
+    for waited, row in zip(*outs):
+        assert all(torch.equal(o, waited[0]) for o in waited + row)
