@@ -14,7 +14,8 @@
 //
 // The keys of a block of queries come from up to five places, each a run of key blocks of 64 rows:
 // pooled rows; kept first positions that lie before the earliest window, cached or of this step; the
-// ring, walked in blocks of its rows as in attention_tc.cu; and the step's own rows.
+// ring, walked in blocks of its rows as in attention_tc.cu; and the step's own rows.  V's rows that no query
+// of the block sees are cleared between copy and product (ta_clear_foreign_rows).
 // The mma.sync kernel that these head sizes took before: 196 us for 2,048 tokens of 16 heads of 128
 // behind a window of 1,024 with pooled blocks; here 62. Three causal prompts of 2,150 tokens in all: 132 -> 50.
 #include "api.h"

@@ -40,7 +40,8 @@
 // nothing visible are masked.  (The mma.sync kernel, which such steps took before: 1,226 us for 2,048
 // tokens of 32 heads of 128 behind a window of 4,096, about 220 here; one layer over a text of 6,001
 // tokens in portions of 2,048 at 7B sizes 4.48 -> 3.48 ms.)
-// Every wait on a barrier is bounded.
+// In every form, V's rows that lie beyond the sequence's own in a block's 64 are cleared between copy and
+// product (ta_clear_foreign_rows).  Every wait on a barrier is bounded.
 #include "api.h"
 #include "attention_tc.cuh"
 
